@@ -24,7 +24,7 @@ EXPORTS = ['jk_plan_create', 'jk_plan_destroy', 'jk_plan_info', 'jk_build',
            'jk_batch_create', 'jk_batch_destroy', 'jk_batch_build', 'jk_batch_sync',
            'jk_batch_counts', 'jk_batch_set_timing', 'jk_batch_class_ms',
            'jk_batch_set_tuning', 'jk_batch_stats', 'jk_last_error', 'jk_grad',
-           'jk_plan_set_jmd']
+           'jk_plan_set_jmd', 'jk_rsqrt']
 
 _lib = None
 
@@ -66,6 +66,7 @@ def lib():
     L.jk_set_timing.argtypes = [vp, c_int]
     L.jk_last_class_ms.argtypes = [vp, ctypes.POINTER(ctypes.c_float), c_int, ip]
     L.jk_fp64_peak.argtypes = [c_int, ctypes.POINTER(ctypes.c_double)]
+    L.jk_rsqrt.argtypes = [c_int, vp, vp, vp, c_int, vp]
     llp = ctypes.POINTER(ctypes.c_longlong)
     ullp = ctypes.POINTER(ctypes.c_ulonglong)
     L.jk_plan_memory.argtypes = [vp, llp, llp]

@@ -634,7 +634,9 @@ static int engine_prepare(Engine &E, std::vector<Item> &items, const Spec &s, ch
     for (int t = 0; t < 2; ++t) {
         const bool on = t < s.nterm;
         E.op_coef[t] = on ? s.coef[t] : 0.0;
-        E.op_inv_om2[t] = on && s.omega[t] > 0 ? 1.0 / (s.omega[t] * s.omega[t]) : 0.0;
+        // (kept finite for a tiny omega, whose operator is 0 in any case)
+        const double om2 = s.omega[t] * s.omega[t];
+        E.op_inv_om2[t] = on && s.omega[t] > 0 ? 1.0 / std::max(om2, 1e-200) : 0.0;
     }
     bool any = false;
     for (const Item &it : items) any = any || it.n_j || it.n_k;
@@ -2193,6 +2195,21 @@ extern "C" int jk_fp64_peak(int device, double *tflops)
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     cudaFree(d_out);
+    return JK_OK;
+}
+
+__global__ void rsqrt_probe(const double *x, double *y, double *z, int n)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) rsqrt_rcp(x[i], y[i], z[i]);
+}
+
+extern "C" int jk_rsqrt(int device, const double *x, double *y, double *z, int n, void *stream)
+{
+    if (!x || !y || !z || n < 1) return fail(JK_ERR_ARG, "jk_rsqrt: null array or n < 1");
+    DeviceGuard g(device);
+    rsqrt_probe<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(x, y, z, n);
+    CK(cudaGetLastError());
     return JK_OK;
 }
 

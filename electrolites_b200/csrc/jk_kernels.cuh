@@ -106,18 +106,6 @@ __device__ __forceinline__ void rys_eval(double x, const double *__restrict__ ch
     }
 }
 
-// 1 / sqrt(a) of a positive, normal a: the hardware's approximation y (about 20
-// bits) and one third-order step, y (1 + e/2 + 3 e^2/8) with e = 1 - a y^2, the
-// first terms of (1 - e)^(-1/2).  No branch for zeros and infinities, which
-// sums of exponents and Boys arguments are not.
-__device__ __forceinline__ double rsqrt_pos(double a)
-{
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-    const double e = fma(-a * y, y, 1.0);
-    return fma(y * e, fma(e, 0.375, 0.5), y);
-}
-
 // Boys functions F_0 .. F_L, F_j = (-1)^j d^j F_0/dx^j, of the order-N (1 or 2)
 // J/K classes from the shared Boys table (BOYS_STRIDE doubles per entry, an
 // odd number of 16-byte slots, so that lanes at different entries spread over
@@ -144,8 +132,10 @@ __device__ __forceinline__ void boys_eval(double x, const double *boys, const do
 {
     constexpr int DEG = boys_degree<N>();
     if (x >= rys_xmax<N>()) {   // F_0 = sqrt(pi / x) / 2, F_(j+1) = (2 j + 1) / (2 x) F_j
-        const double ix = rsqrt_pos(x);
-        const double hx = __ldg(tab + RYS_LARGEX_OFF) * (ix * ix);     // 1 / (2 x)
+        double ix, rx;
+        // (an overflowed distance: x <= 1.1e300 by its high word, F ~ 0)
+        rsqrt_rcp(__hiloint2double(min(__double2hiint(x), 0x7e3a0000), __double2loint(x)), ix, rx);
+        const double hx = __ldg(tab + RYS_LARGEX_OFF) * rx;            // 1 / (2 x)
         f[0] = __ldg(tab + RYS_LARGEX_OFF + RYS_NMAX * RYS_NMAX) * ix;
 #pragma unroll
         for (int j = 0; j < L; ++j) f[j + 1] = f[j] * ((2 * j + 1) * hx);
@@ -757,8 +747,8 @@ __device__ __forceinline__ void reg_accum(const ClassArgs &A, const PlanView &V,
                     // inv_om2 = 1/omega^2 > 0: the long-range erf(omega r)/r
                     // operator, whose Rys quadrature is the Coulomb one with
                     // a_ij + a_kl replaced by a_ij + a_kl + a_ij a_kl / omega^2
-                    const double rs = rsqrt_pos(fma(aij * akl, io2, aij + akl));
-                    const double is = rs * rs;
+                    double rs, is;
+                    rsqrt_rcp(fma(aij * akl, io2, aij + akl), rs, is);
                     const double rr = fma(PQx, PQx, fma(PQy, PQy, PQz * PQz));
                     const double x = aij * akl * is * rr;
                     const double pref = s23.x * kq * rs;

@@ -214,6 +214,10 @@ int jk_last_class_ms(jk_plan *plan, float *ms, int ncounts, int *launches);
  */
 int jk_fp64_peak(int device, double *tflops);
 
+/* The kernels' y = 1/sqrt(x) and z = 1/x of n positive numbers on the device
+ * (for comparing them with others). */
+int jk_rsqrt(int device, const double *x, double *y, double *z, int n, void *stream);
+
 /* Schwarz bounds q[nbas][nbas] (host, float, -inf for pairs below the
  * plan's range), in the caller's shell numbering when no shell has a
  * general contraction. */

@@ -433,3 +433,40 @@ def test_mixed_form_team_classes(torch, oracle, seed):
     assert abs(ej - mej) <= 1e-7 and abs(ek - mek) <= 1e-7
     opt.get_jk(d, 1)
     assert sum(c[2] for c in opt.class_counts(with_f32=True).values()) == 0
+
+
+@pytest.mark.parametrize('w', [1e-140, 1e-160, 1e-300])
+def test_tiny_omega(torch, w):
+    """erf(w r)/r <= 2 w / sqrt(pi) for every r: J, K and forces of so small a
+    w vanish (the engine takes w as 1e-100 at least), also where 1/w^2 is past
+    the largest double, and mixing them in leaves the Coulomb part as it is."""
+    from electrolites_b200.jk import VHFOpt
+    mol = all_class_mol()
+    opt = VHFOpt(mol, TOL).build()
+    d = torch.as_tensor(densities(mol, 'random', 1, 1, np.random.default_rng(4)), device='cuda')
+    for v in (*opt.get_jk(d, 1, omega=w), opt.get_jk(d, 1, omega=w, with_k=False)[0],
+              opt.jk_energy_per_atom(d, 1.0, 1.0, w)):
+        assert float(v.abs().max()) <= 1e-90      # false for NaN
+    vj, vk = opt.get_jk(d, 1)
+    assert float((opt.get_k(d, 1, omega=w, lr_factor=0.5, sr_factor=1.0) - vk).abs().max()) <= ATOL
+    sj, sk = opt.get_jk(d, 1, omega=-w)
+    assert float((sj - vj).abs().max()) <= ATOL and float((sk - vk).abs().max()) <= ATOL
+
+
+def test_reciprocal_square_root(torch):
+    """The kernels' 1/sqrt and 1/x over the arguments they give them (sums of
+    exponents, those of the long-range operator, Boys arguments) against CUDA's.
+    Both are one rounded fma, u = 2^-53, after corrections of 2^-19 whose own
+    roundings are 2^-72 and whose series leave 2^-57; CUDA's 1/sqrt is within 2 u,
+    its division and each quotient here within u."""
+    from electrolites_b200 import _lib
+    u = 2.0 ** -53
+    rng = np.random.default_rng(1)
+    x = np.concatenate([10.0 ** rng.uniform(-300, 300, 200000), 10.0 ** rng.uniform(-3, 6, 400000),
+                        rng.uniform(1.0, 4.0, 400000), [1e-300, 1.0, 2.0, 4.0, 1e300]])
+    x = torch.as_tensor(x, device='cuda')
+    y, z = torch.empty_like(x), torch.empty_like(x)
+    _lib.check(_lib.lib().jk_rsqrt(0, x.data_ptr(), y.data_ptr(), z.data_ptr(), len(x), None), 'jk_rsqrt')
+    torch.cuda.synchronize()
+    assert float((y / torch.rsqrt(x) - 1).abs().max()) <= 4.2 * u
+    assert float((z / (1.0 / x) - 1).abs().max()) <= 3.2 * u
