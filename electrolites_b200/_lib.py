@@ -24,7 +24,7 @@ EXPORTS = ['jk_plan_create', 'jk_plan_destroy', 'jk_plan_info', 'jk_build',
            'jk_batch_create', 'jk_batch_destroy', 'jk_batch_build', 'jk_batch_sync',
            'jk_batch_counts', 'jk_batch_set_timing', 'jk_batch_class_ms',
            'jk_batch_set_tuning', 'jk_batch_stats', 'jk_last_error', 'jk_grad',
-           'jk_plan_set_jmd', 'jk_rsqrt']
+           'jk_plan_set_jmd', 'jk_rsqrt', 'jk_plan_stats']
 
 _lib = None
 
@@ -70,6 +70,7 @@ def lib():
     llp = ctypes.POINTER(ctypes.c_longlong)
     ullp = ctypes.POINTER(ctypes.c_ulonglong)
     L.jk_plan_memory.argtypes = [vp, llp, llp]
+    L.jk_plan_stats.argtypes = [vp, ip, ip]
     L.jk_plan_set_shard.argtypes = [vp, c_int, c_int]
     L.jk_plan_set_tol.argtypes = [vp, c_double]
     L.jk_plan_set_jengine.argtypes = [vp, c_int]

@@ -238,6 +238,7 @@ struct Engine {
     cudaStream_t gstream = nullptr;
     std::vector<char> gkey, gkey_last;
     int grepeat = 0, glaunches = 0;
+    int last_replayed = 0, last_captured = 0;   // the last build: a replay, a capture
     char *ws = nullptr;             // workspace of the prepared build
     size_t acc_bytes = 0;           // accumulators at its start (cleared per build)
 };
@@ -669,7 +670,8 @@ static int engine_prepare(Engine &E, std::vector<Item> &items, const Spec &s, ch
             v.dm_cond = it.dmc;
             v.scr = p->d_scr + p->pc_off[B];
             v.dkl = it.dkl ? it.dkl + p->pc_off[B] : nullptr;
-            v.dmK = it.DN ? it.DN : it.dm;
+            // (no K: none, the caller's address is no part of the launch key)
+            v.dmK = !it.n_k ? nullptr : it.DN ? it.DN : it.dm;
             v.dmKT = it.DT;
             v.dmK2 = it.dmK2;
             v.dsJ = it.dsJ;
@@ -1177,6 +1179,9 @@ static int engine_run(Engine &E, cudaStream_t st)
         E.gexec = exec;
         E.gkey = key;
         E.glaunches = E.launches;
+        E.last_captured = 1;
+    } else {
+        E.last_replayed = 1;
     }
     E.gkey_last = key;   // (builds of another shape in between start their count again)
     E.grepeat = 0;
@@ -1191,6 +1196,7 @@ static int engine_build(Engine &E, std::vector<Item> &items, const Spec &s, cuda
                         char *ws_ext, size_t ws_ext_size, bool no_alloc, const char *who,
                         bool plan = true)
 {
+    E.last_replayed = E.last_captured = 0;
     RC(engine_prepare(E, items, s, ws_ext, ws_ext_size, no_alloc, who));
     RC(engine_upload(E, st));
     RC(plan && !ws_ext ? engine_run(E, st) : engine_launch(E, st, E.timing));
@@ -1715,6 +1721,14 @@ extern "C" int jk_plan_memory(const jk_plan *plan, long long *table_bytes, long 
         *table_bytes = (long long)(plan->table_bytes + row_bytes(plan->eng.max_rows) +
                                    plan->eng.blob_cap);
     if (workspace_bytes) *workspace_bytes = (long long)(plan->eng.ws_size + plan->io_size);
+    return JK_OK;
+}
+
+extern "C" int jk_plan_stats(const jk_plan *plan, int *graph_replayed, int *graph_captured)
+{
+    if (!plan) return fail(JK_ERR_ARG, "jk_plan_stats: plan is NULL");
+    if (graph_replayed) *graph_replayed = plan->eng.last_replayed;
+    if (graph_captured) *graph_captured = plan->eng.last_captured;
     return JK_OK;
 }
 

@@ -329,6 +329,14 @@ class VHFOpt:
                    'jk_plan_memory')
         return t.value, w.value
 
+    def stats(self):
+        """{'graph_replayed', 'graph_captured'} of the last build."""
+        r = ctypes.c_int()
+        c = ctypes.c_int()
+        _lib.check(_lib.lib().jk_plan_stats(self.plan, ctypes.byref(r), ctypes.byref(c)),
+                   'jk_plan_stats')
+        return {'graph_replayed': bool(r.value), 'graph_captured': bool(c.value)}
+
     def q_cond(self):
         nb = len(self._bas)
         q = np.zeros((nb, nb), dtype=np.float32)

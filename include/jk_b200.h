@@ -228,6 +228,11 @@ int jk_plan_q_cond(const jk_plan *plan, float *q_host, int nbas);
 int jk_plan_memory(const jk_plan *plan, long long *table_bytes,
                    long long *workspace_bytes);
 
+/* Whether the plan's last build replayed the graph of an earlier one, or
+ * captured it (a small plan's third build of one kind in a row; either way
+ * the build ran as a graph). */
+int jk_plan_stats(const jk_plan *plan, int *graph_replayed, int *graph_captured);
+
 /*
  * Multi-GPU sharding of a plan's builds: with size > 1 a build evaluates
  * only the tasks t = rank + size * n of every class's task list, so the

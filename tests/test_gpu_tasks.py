@@ -126,3 +126,40 @@ def test_repeated_builds_of_changing_kinds(torch):
             assert (a is None) == (b is None)
             if a is not None:
                 assert float((a - b).abs().max()) <= ATOL
+
+
+def _once(o, k, d):
+    """One call of kind k: the plan's outputs that there are."""
+    if k == 'grad':
+        return (o.jk_energy_per_atom(d, 1.0, 0.3),)
+    if k == 'rsh':
+        return (o.get_k(d, omega=0.4, lr_factor=1.0, sr_factor=0.2),)
+    if k == 'j':
+        return (o.get_j(d),)
+    return o.get_jk(d, 0 if k == 'general' else 1)
+
+
+@pytest.mark.parametrize('kind', ['jk', 'j', 'general', 'grad', 'rsh'])
+def test_graph_replay_with_moving_densities(torch, kind):
+    """The third build of a kind captures, the later ones replay, with every
+    density at an address of its own; two streams in turn share the graph.
+    A replay gives what a fresh plan's direct launches give."""
+    from electrolites_b200.jk import VHFOpt
+    mol = clusters.water_mole(2, 4.2, 17)
+    opt = VHFOpt(mol, TOL).build()
+    base = clusters.atomic_density(mol, 3)
+    rng = np.random.default_rng(6)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    kept = []
+    for n in range(8):
+        p = 1e-2 * rng.standard_normal((1,) + base.shape)
+        d = torch.as_tensor(base + (p if kind == 'general' else p + p.transpose(0, 2, 1)), device='cuda')
+        torch.cuda.synchronize()
+        with torch.cuda.stream(streams[n % 2]):
+            got = _once(opt, kind, d)
+        assert opt.stats() == {'graph_replayed': n > 2, 'graph_captured': n == 2}
+        kept.append((d, got))
+        fresh = VHFOpt(mol, TOL).build()
+        for a, b in zip(got, _once(fresh, kind, d)):
+            assert float((a - b).abs().max()) <= ATOL
+        assert not any(fresh.stats().values())
