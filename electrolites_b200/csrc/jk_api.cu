@@ -1108,12 +1108,18 @@ static int engine_launch(Engine &E, cudaStream_t st, bool timing, int streams = 
     return JK_OK;
 }
 
+// The end of a build on the stream.  A build that the caller captures into a graph
+// of its own ends when that graph has run, which only the caller can wait for:
+// its record would be an event that no host call may wait on.
 static int engine_finish(Engine &E, cudaStream_t st)
 {
+    E.last_stream = st;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+    if (cap != cudaStreamCaptureStatusNone) return JK_OK;
     CK(cudaEventRecord(E.done_ev, st));
     E.done_ev_rec = true;
     E.done_stream = st;
-    E.last_stream = st;
     return JK_OK;
 }
 

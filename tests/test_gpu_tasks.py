@@ -163,3 +163,33 @@ def test_graph_replay_with_moving_densities(torch, kind):
         for a, b in zip(got, _once(fresh, kind, d)):
             assert float((a - b).abs().max()) <= ATOL
         assert not any(fresh.stats().values())
+
+
+def test_build_in_the_callers_graph(torch):
+    """A build captured into the caller's own graph: its replays give the J/K of
+    the densities then in the buffers, jk_sync waits for them, and the plan's
+    ordinary builds go on."""
+    from electrolites_b200.jk import VHFOpt
+    mol = clusters.water_mole(2, 4.2, 17)
+    opt = VHFOpt(mol, TOL).build()
+    base = torch.as_tensor(clusters.atomic_density(mol, 3)[None], device='cuda')
+    dm, vj, vk = base.clone(), torch.empty_like(base), torch.empty_like(base)
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for _ in range(2):                   # warm: buffers, descriptors, kernel attributes
+        opt.build_jk_async(dm, 1, vj=vj, vk=vk, stream=st)
+    opt.sync(st)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=st):
+        opt.build_jk_async(dm, 1, vj=vj, vk=vk, stream=st)
+    for f in (1.0, 0.7):
+        dm.copy_(f * base)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(st):
+            g.replay()
+        opt.sync(st)
+        rj, rk = VHFOpt(mol, TOL).build().get_jk(dm, 1)
+        assert float((vj - rj).abs().max()) <= ATOL and float((vk - rk).abs().max()) <= ATOL
+    aj, ak = opt.get_jk(base, 1)
+    assert float((0.7 * aj - rj).abs().max()) <= ATOL and float((0.7 * ak - rk).abs().max()) <= ATOL
+    del g
