@@ -1304,6 +1304,7 @@ static void free_plan(jk_plan *p)
     cudaFree(p->d_ao_plan);
     cudaFree(p->d_sh_ao);
     cudaFree(p->d_sh_nf);
+    cudaFree(p->d_sh_atom);
     cudaFree(p->d_io);
     engine_free(p->eng);
 }

@@ -80,6 +80,18 @@ def test_library_exports_every_header_symbol():
     assert set(syms) <= set(_lib.EXPORTS)
 
 
+def test_a_destroyed_plan_frees_every_device_table():
+    """Every device pointer that a plan owns is freed with it (a scan over
+    geometries makes and destroys a plan per step)."""
+    src = open(os.path.join(ROOT, 'electrolites_b200', 'csrc', 'jk_api.cu')).read()
+    plan = re.search(r'^struct jk_plan \{\n(.*?)^\};', src, re.M | re.S).group(1)
+    free = re.search(r'^static void free_plan\(.*?^\}', src, re.M | re.S).group(0)
+    tables = re.findall(r'\*(d_\w+) = nullptr', plan)
+    assert 'd_pairs' in tables and 'd_sh_atom' in tables
+    for t in tables:
+        assert f'cudaFree(p->{t});' in free, t
+
+
 def test_library_errors_without_device_or_bad_args():
     """Argument errors come back as codes with a message; no silent path."""
     from electrolites_b200 import _lib
