@@ -153,6 +153,12 @@ struct ClassTune {
 // lose: (H2O)_17 gradient, 29 000 task rows, 26.8 -> 28.0 ms)
 #define JK_GRAPH_STREAMS 12
 
+// Side streams of a build and the events that fork and join them.
+struct StreamSet {
+    cudaStream_t side[JK_GRAPH_STREAMS] = {};
+    cudaEvent_t fork = nullptr, join[JK_GRAPH_STREAMS] = {};
+};
+
 struct Engine {
     int device = 0, num_sms = 148;
     // nuclear-gradient build (grad != null): its sums in the workspace, copied
@@ -167,11 +173,8 @@ struct Engine {
     // (max_rows each), chunks per scan tile (row_tiles(max_rows))
     int *d_rows = nullptr;
     long long max_rows = 0;
-    // class streams besides the build's (those past JK_CLASS_STREAMS made when a
-    // graph is captured)
-    cudaStream_t side[JK_GRAPH_STREAMS - 1] = {};
-    cudaEvent_t ev_fork = nullptr;
-    cudaEvent_t ev_join[JK_GRAPH_STREAMS - 1] = {};
+    bool in_capture = false;        // the caller captures the stream of this build
+    StreamSet own_streams;          // of such builds (engine_direct)
     int *d_chunk = nullptr;         // task size per class
     // cleared per build, one buffer: quartets, primitive quartets, FP32
     // quartets and candidates per class, then a task counter per class launch
@@ -235,7 +238,6 @@ struct Engine {
     // the launch stream of a plan's small builds as a graph (engine_run): the
     // key it was captured for, the key of the last build, builds in a row with it
     cudaGraphExec_t gexec = nullptr;
-    cudaStream_t gstream = nullptr;
     std::vector<char> gkey, gkey_last;
     int grepeat = 0, glaunches = 0;
     int last_replayed = 0, last_captured = 0;   // the last build: a replay, a capture
@@ -283,7 +285,6 @@ struct jk_plan {
 
 struct jk_batch {
     Engine eng;
-    cudaStream_t cap_stream = nullptr;   // capture stream of the graph
     cudaGraphExec_t gexec = nullptr;
     std::vector<char> graph_blob;
     unsigned graph_alloc_gen = 0, graph_tune_gen = 0;
@@ -313,13 +314,59 @@ static size_t stat_bytes(int ncounters)
     return 4 * JK_NCLASSES * sizeof(unsigned long long) + ncounters * sizeof(int);
 }
 
-static int class_streams(Engine &E, int n)
+// the n - 1 side streams of a build on n
+static int make_streams(StreamSet &ss, int n)
 {
+    if (!ss.fork) CK(cudaEventCreateWithFlags(&ss.fork, cudaEventDisableTiming));
     for (int s = 0; s < n - 1; ++s) {
-        if (!E.side[s]) CK(cudaStreamCreateWithFlags(&E.side[s], cudaStreamNonBlocking));
-        if (!E.ev_join[s]) CK(cudaEventCreateWithFlags(&E.ev_join[s], cudaEventDisableTiming));
+        if (!ss.side[s]) CK(cudaStreamCreateWithFlags(&ss.side[s], cudaStreamNonBlocking));
+        if (!ss.join[s]) CK(cudaEventCreateWithFlags(&ss.join[s], cudaEventDisableTiming));
     }
     return JK_OK;
+}
+
+static void free_streams(StreamSet &ss)
+{
+    if (ss.fork) cudaEventDestroy(ss.fork);
+    for (int s = 0; s < JK_GRAPH_STREAMS; ++s) {
+        if (ss.side[s]) cudaStreamDestroy(ss.side[s]);
+        if (ss.join[s]) cudaEventDestroy(ss.join[s]);
+    }
+    ss = StreamSet();
+}
+
+// The side streams of all plans and batches of a device, kept until exit: a
+// stream takes half a megabyte of device memory and 50 us to make.  Builds on
+// one stream of the caller run one after another whatever side streams they
+// use, so each of the caller's first JK_STREAM_SETS streams has a set, and
+// later ones share them (which orders their builds, nothing else).  Set 0 is
+// made with the device's first plan, for the default stream and for
+// allocation-free builds, which may make none.  capture: captures of graphs,
+// whose nodes keep no stream.  A set's mutex is held while a build is put on it.
+#define JK_STREAM_SETS 8
+struct DeviceStreams {
+    struct Shared : StreamSet {
+        std::mutex mutex;
+    };
+    std::mutex mutex;               // of the list
+    int n = 1, next = 0;            // sets in use, the next to be shared
+    cudaStream_t of[JK_STREAM_SETS] = {};
+    Shared set[JK_STREAM_SETS], capture;
+};
+static DeviceStreams g_streams[JK_MAX_DEVICES];
+
+static DeviceStreams::Shared &shared_streams(int device, cudaStream_t st)
+{
+    DeviceStreams &D = g_streams[device];
+    std::lock_guard<std::mutex> lock(D.mutex);
+    for (int k = 0; k < D.n; ++k)
+        if (D.of[k] == st) return D.set[k];
+    if (D.n < JK_STREAM_SETS) {
+        D.of[D.n] = st;
+        return D.set[D.n++];
+    }
+    D.next = (D.next + 1) % JK_STREAM_SETS;
+    return D.set[D.next];
 }
 
 static int engine_init(Engine &E, int device)
@@ -337,8 +384,7 @@ static int engine_init(Engine &E, int device)
     E.h_error[0] = E.h_error[1] = 0;
     CK(cudaEventCreateWithFlags(&E.blob_ev, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&E.done_ev, cudaEventDisableTiming));
-    CK(cudaEventCreateWithFlags(&E.ev_fork, cudaEventDisableTiming));
-    return class_streams(E, JK_CLASS_STREAMS);
+    return JK_OK;
 }
 
 static void engine_free(Engine &E)
@@ -352,14 +398,9 @@ static void engine_free(Engine &E)
     if (E.h_blob) cudaFreeHost(E.h_blob);
     if (E.blob_ev) cudaEventDestroy(E.blob_ev);
     if (E.done_ev) cudaEventDestroy(E.done_ev);
-    if (E.ev_fork) cudaEventDestroy(E.ev_fork);
-    for (int s = 0; s < JK_GRAPH_STREAMS - 1; ++s) {
-        if (E.side[s]) cudaStreamDestroy(E.side[s]);
-        if (E.ev_join[s]) cudaEventDestroy(E.ev_join[s]);
-    }
+    free_streams(E.own_streams);
     for (auto &e : E.ev) cudaEventDestroy(e);
     if (E.gexec) cudaGraphExecDestroy(E.gexec);
-    if (E.gstream) cudaStreamDestroy(E.gstream);
     E = Engine();
 }
 
@@ -978,10 +1019,12 @@ static int jx_pairs(Engine &E, cudaStream_t st, bool post)
     return JK_OK;
 }
 
-// The launch stream of a prepared build (stream operations only, so that it
-// can be captured).
-static int engine_launch(Engine &E, cudaStream_t st, bool timing, int streams = JK_CLASS_STREAMS)
+// The launch stream of a prepared build on `streams` streams (stream operations
+// only, so that it can be captured).
+static int engine_launch(Engine &E, cudaStream_t st, bool timing, StreamSet &ss,
+                         int streams = JK_CLASS_STREAMS)
 {
+    RC(make_streams(ss, streams));
     E.launches = 0;
     if (timing) std::fill(E.ev_used.begin(), E.ev_used.end(), 0);
     const TileOp *d_pre = (const TileOp *)(E.d_blob + E.off_pre);
@@ -990,9 +1033,9 @@ static int engine_launch(Engine &E, cudaStream_t st, bool timing, int streams = 
     if (E.acc_bytes) CK(cudaMemsetAsync(E.ws, 0, E.acc_bytes, st));
     // two chains side by side: the densities the class kernels read (on the
     // first side stream), and the screening table with the task list
-    cudaStream_t dst = E.side[0];
-    CK(cudaEventRecord(E.ev_fork, st));
-    CK(cudaStreamWaitEvent(dst, E.ev_fork, 0));
+    cudaStream_t dst = ss.side[0];
+    CK(cudaEventRecord(ss.fork, st));
+    CK(cudaStreamWaitEvent(dst, ss.fork, 0));
     if (E.npre) {
         tile_op_kernel<<<(unsigned)E.pre_tiles, dim3(32, 8), 0, dst>>>(d_pre, E.npre);
         CK(cudaGetLastError());
@@ -1005,7 +1048,7 @@ static int engine_launch(Engine &E, cudaStream_t st, bool timing, int streams = 
         E.launches++;
     }
     if (E.jx) RC(jx_pairs(E, dst, false));   // x-space densities of every pair
-    CK(cudaEventRecord(E.ev_join[0], dst));
+    CK(cudaEventRecord(ss.join[0], dst));
     dm_cond_kernel<<<(unsigned)E.cond_blocks, dim3(16, 16), 0, st>>>(d_cond, E.nitems);
     CK(cudaGetLastError());
     E.launches++;
@@ -1042,7 +1085,7 @@ static int engine_launch(Engine &E, cudaStream_t st, bool timing, int streams = 
         CK(cudaGetLastError());
         E.launches += 2;
     }
-    CK(cudaStreamWaitEvent(st, E.ev_join[0], 0));   // the densities
+    CK(cudaStreamWaitEvent(st, ss.join[0], 0));   // the densities
     char msg[256] = {0};
     LaunchCfg cfg;
     cfg.device = E.device;
@@ -1056,10 +1099,10 @@ static int engine_launch(Engine &E, cudaStream_t st, bool timing, int streams = 
     const int ns = timing && E.timing_mode == 1 ? 1 : streams;
     cudaStream_t cs[JK_GRAPH_STREAMS];
     cs[0] = st;
-    if (ns > 1) CK(cudaEventRecord(E.ev_fork, st));
+    if (ns > 1) CK(cudaEventRecord(ss.fork, st));
     for (int s = 1; s < ns; ++s) {
-        cs[s] = E.side[s - 1];
-        CK(cudaStreamWaitEvent(cs[s], E.ev_fork, 0));
+        cs[s] = ss.side[s - 1];
+        CK(cudaStreamWaitEvent(cs[s], ss.fork, 0));
     }
     int nactive = 0;
     for (int c = 0; c < JK_NCLASSES; ++c) {
@@ -1089,8 +1132,8 @@ static int engine_launch(Engine &E, cudaStream_t st, bool timing, int streams = 
     }
     // join the class streams back into the build's stream
     for (int s = 1; s < ns; ++s) {
-        CK(cudaEventRecord(E.ev_join[s - 1], cs[s]));
-        CK(cudaStreamWaitEvent(st, E.ev_join[s - 1], 0));
+        CK(cudaEventRecord(ss.join[s - 1], cs[s]));
+        CK(cudaStreamWaitEvent(st, ss.join[s - 1], 0));
     }
     if (E.grad && E.grad_plan->npairs) {
         const int np = (int)E.grad_plan->npairs;
@@ -1108,15 +1151,53 @@ static int engine_launch(Engine &E, cudaStream_t st, bool timing, int streams = 
     return JK_OK;
 }
 
+static bool capturing(cudaStream_t st)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) == cudaSuccess) return cap != cudaStreamCaptureStatusNone;
+    cudaGetLastError();   // the default stream while another one is being captured
+    return true;
+}
+
+// engine_launch on the device's side streams.  Those of a build that the caller
+// captures would be part of the caller's graph until its capture ends, so such
+// a build takes streams of the engine's own.  no_alloc: set 0, which is there.
+static int engine_direct(Engine &E, cudaStream_t st, bool no_alloc = false)
+{
+    if (E.in_capture) return engine_launch(E, st, E.timing, E.own_streams);
+    DeviceStreams::Shared &ss = no_alloc ? g_streams[E.device].set[0] : shared_streams(E.device, st);
+    std::lock_guard<std::mutex> lock(ss.mutex);
+    return engine_launch(E, st, E.timing, ss);
+}
+
+// the launches of a prepared build captured into an executable graph
+static int engine_capture(Engine &E, int streams, cudaGraphExec_t *exec)
+{
+    RC(engine_configure(E));
+    DeviceStreams::Shared &ss = g_streams[E.device].capture;
+    std::lock_guard<std::mutex> lock(ss.mutex);
+    RC(make_streams(ss, streams + 1));
+    const cudaStream_t st = ss.side[streams - 1];   // the build's, beside its side streams
+    CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
+    const int rc = engine_launch(E, st, false, ss, streams);
+    cudaGraph_t graph = nullptr;
+    const cudaError_t ce = cudaStreamEndCapture(st, &graph);
+    cudaError_t ie = cudaSuccess;
+    if (rc == JK_OK && ce == cudaSuccess) ie = cudaGraphInstantiate(exec, graph, 0);
+    if (graph) cudaGraphDestroy(graph);
+    RC(rc);
+    CK(ce);
+    CK(ie);
+    return JK_OK;
+}
+
 // The end of a build on the stream.  A build that the caller captures into a graph
 // of its own ends when that graph has run, which only the caller can wait for:
 // its record would be an event that no host call may wait on.
 static int engine_finish(Engine &E, cudaStream_t st)
 {
     E.last_stream = st;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
-    if (cap != cudaStreamCaptureStatusNone) return JK_OK;
+    if (E.in_capture) return JK_OK;
     CK(cudaEventRecord(E.done_ev, st));
     E.done_ev_rec = true;
     E.done_stream = st;
@@ -1154,32 +1235,17 @@ static std::vector<char> launch_key(const Engine &E)
 
 static int engine_run(Engine &E, cudaStream_t st)
 {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
-    if (E.timing || E.nrows > JK_GRAPH_ROWS || cudaStreamIsCapturing(st, &cap) != cudaSuccess ||
-        cap != cudaStreamCaptureStatusNone) {
-        cudaGetLastError();
-        return engine_launch(E, st, E.timing);
-    }
+    if (E.timing || E.nrows > JK_GRAPH_ROWS || E.in_capture) return engine_direct(E, st);
     std::vector<char> key = launch_key(E);
     if (!E.gexec || key != E.gkey) {
         E.grepeat = key == E.gkey_last ? E.grepeat + 1 : 0;
         E.gkey_last = key;
-        if (E.grepeat < 2) return engine_launch(E, st, false);
-        if (!E.gstream) CK(cudaStreamCreateWithFlags(&E.gstream, cudaStreamNonBlocking));
-        RC(class_streams(E, JK_GRAPH_STREAMS));
-        RC(engine_configure(E));
-        CK(cudaStreamBeginCapture(E.gstream, cudaStreamCaptureModeRelaxed));
-        const int rc = engine_launch(E, E.gstream, false, JK_GRAPH_STREAMS);
-        cudaGraph_t graph = nullptr;
-        const cudaError_t ce = cudaStreamEndCapture(E.gstream, &graph);
+        if (E.grepeat < 2) return engine_direct(E, st);
         cudaGraphExec_t exec = nullptr;
-        const cudaError_t ie = rc == JK_OK && ce == cudaSuccess ? cudaGraphInstantiate(&exec, graph, 0)
-                                                               : cudaErrorUnknown;
-        if (graph) cudaGraphDestroy(graph);
-        if (ie != cudaSuccess) {   // as before, call by call
+        if (engine_capture(E, JK_GRAPH_STREAMS, &exec) != JK_OK) {   // as before, call by call
             cudaGetLastError();
             E.gkey_last.clear();
-            return engine_launch(E, st, false);
+            return engine_direct(E, st);
         }
         if (E.gexec) cudaGraphExecDestroy(E.gexec);
         E.gexec = exec;
@@ -1203,9 +1269,13 @@ static int engine_build(Engine &E, std::vector<Item> &items, const Spec &s, cuda
                         bool plan = true)
 {
     E.last_replayed = E.last_captured = 0;
+    E.in_capture = capturing(st);
     RC(engine_prepare(E, items, s, ws_ext, ws_ext_size, no_alloc, who));
     RC(engine_upload(E, st));
-    RC(plan && !ws_ext ? engine_run(E, st) : engine_launch(E, st, E.timing));
+    if (plan && !ws_ext)
+        RC(engine_run(E, st));
+    else
+        RC(engine_direct(E, st, no_alloc));
     if (E.grad_out)
         CK(cudaMemcpyAsync(E.grad_out, E.grad, E.grad_bytes, cudaMemcpyDeviceToDevice, st));
     return engine_finish(E, st);
@@ -1409,6 +1479,11 @@ static int plan_create(const int *atm, int natm, const int *bas, int nbas_user, 
     p->nbas_user = nbas_user;
     p->natm = natm;
     RC(engine_init(p->eng, device));
+    {
+        DeviceStreams::Shared &ss = g_streams[device].set[0];
+        std::lock_guard<std::mutex> lock(ss.mutex);
+        RC(make_streams(ss, JK_CLASS_STREAMS));
+    }
 
     // ---- shells (general contractions expanded, contraction-major) ----
     std::vector<ShellDev> shells;
@@ -2016,8 +2091,6 @@ extern "C" int jk_batch_create(int device, jk_batch **out)
     DeviceGuard g(device);
     jk_batch *b = new jk_batch();
     int rc = engine_init(b->eng, device);
-    if (rc == JK_OK && cudaStreamCreateWithFlags(&b->cap_stream, cudaStreamNonBlocking) != cudaSuccess)
-        rc = fail(JK_ERR_CUDA, "jk_batch_create: cannot create the capture stream");
     if (rc != JK_OK) {
         engine_free(b->eng);
         delete b;
@@ -2033,7 +2106,6 @@ extern "C" int jk_batch_destroy(jk_batch *batch)
     DeviceGuard g(batch->eng.device);
     engine_idle(batch->eng);
     if (batch->gexec) cudaGraphExecDestroy(batch->gexec);
-    if (batch->cap_stream) cudaStreamDestroy(batch->cap_stream);
     engine_free(batch->eng);
     delete batch;
     return JK_OK;
@@ -2066,6 +2138,7 @@ extern "C" int jk_batch_build(jk_batch *batch, jk_plan *const *plans, int nplans
         batch->warmed = true;
         return JK_OK;
     }
+    E.in_capture = capturing(st);
     RC(engine_prepare(E, items, s, nullptr, 0, false, "jk_batch_build"));
     const int spec[4] = {hermi, with_j, with_k, E.shard_rank * 65536 + E.shard_size};
     const bool same = batch->gexec && E.blob == batch->graph_blob && E.blob_dev == batch->graph_blob &&
@@ -2078,19 +2151,7 @@ extern "C" int jk_batch_build(jk_batch *batch, jk_plan *const *plans, int nplans
             cudaGraphExecDestroy(batch->gexec);
             batch->gexec = nullptr;
         }
-        RC(engine_configure(E));
-        CK(cudaStreamBeginCapture(batch->cap_stream, cudaStreamCaptureModeRelaxed));
-        const int rc = engine_launch(E, batch->cap_stream, false);
-        cudaGraph_t graph = nullptr;
-        const cudaError_t ce = cudaStreamEndCapture(batch->cap_stream, &graph);
-        if (rc != JK_OK) {
-            if (graph) cudaGraphDestroy(graph);
-            return rc;
-        }
-        CK(ce);
-        const cudaError_t ie = cudaGraphInstantiate(&batch->gexec, graph, 0);
-        cudaGraphDestroy(graph);
-        CK(ie);
+        RC(engine_capture(E, JK_CLASS_STREAMS, &batch->gexec));
         batch->graph_blob = E.blob;
         batch->graph_alloc_gen = E.alloc_gen;
         batch->graph_tune_gen = E.tune_gen;

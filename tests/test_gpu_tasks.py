@@ -193,3 +193,61 @@ def test_build_in_the_callers_graph(torch):
     aj, ak = opt.get_jk(base, 1)
     assert float((0.7 * aj - rj).abs().max()) <= ATOL and float((0.7 * ak - rk).abs().max()) <= ATOL
     del g
+
+
+def test_plans_hold_no_streams(torch):
+    """A plan takes its tables and little more of the device (a stream takes
+    half a megabyte): 64 plans of one water, built in a batch and each alone,
+    stay below a megabyte each."""
+    from electrolites_b200.batch import JKBatch
+    from electrolites_b200.jk import VHFOpt
+    mol = clusters.water_mole(1, 3.0, 7)
+    d = torch.as_tensor(clusters.atomic_density(mol, 3)[None], device='cuda')
+    batch = JKBatch()
+    first = VHFOpt(mol, TOL).build()
+    out = [torch.empty((64,) + d.shape, dtype=d.dtype, device='cuda') for _ in range(2)]
+    batch.build([first], [d], 1)
+    vj, vk = first.get_jk(d, 1)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    opts = [VHFOpt(mol, TOL).build() for _ in range(64)]
+    batch.build(opts, [d] * 64, 1, vj=list(out[0]), vk=list(out[1]))
+    for o in opts:
+        o.build_jk_async(d, 1, vj=vj, vk=vk)
+        o.sync()
+    assert free - torch.cuda.mem_get_info()[0] < 64 << 20
+    assert float((out[1][63] - vk).abs().max()) <= ATOL
+
+
+def test_builds_of_many_streams_and_threads(torch):
+    """More streams than the device has sets of side streams, from four threads
+    at a time, each plan on its own stream: every build is its plan's."""
+    import threading
+
+    from electrolites_b200.jk import VHFOpt
+    work = []
+    for k in range(12):
+        mol = clusters.water_mole(1 + k % 3, 4.5, 40 + k)
+        d = torch.as_tensor(clusters.atomic_density(mol, k)[None], device='cuda')
+        work.append((VHFOpt(mol, TOL).build(), d, VHFOpt(mol, TOL).build().get_jk(d, 1), torch.cuda.Stream()))
+    torch.cuda.synchronize()
+    bad = []
+
+    def some(mine):
+        for _ in range(6):               # direct builds, a capture, replays
+            got = []
+            for opt, d, _, st in mine:
+                vj, vk = torch.empty_like(d), torch.empty_like(d)
+                opt.build_jk_async(d, 1, vj=vj, vk=vk, stream=st)
+                got.append((vj, vk))
+            for (opt, _, ref, st), g in zip(mine, got):
+                opt.sync(st)
+                bad.extend(float((a - b).abs().max()) for a, b in zip(g, ref)
+                           if not float((a - b).abs().max()) <= ATOL)
+
+    threads = [threading.Thread(target=some, args=(work[k::4],)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
