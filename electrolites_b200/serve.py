@@ -78,15 +78,21 @@ def matrix_bytes(nao: int, nbas: int, n_dm: int, incremental: bool = False) -> i
     """Device bytes of a request's matrices: densities, J, K, and its share
     of the build workspace (half-J/K accumulators, symmetrised densities,
     the K densities in the plan's AO order and their pair-interleaved copy,
-    screening table) for hermi = 1; incremental mode keeps four more (the
-    previous density, the density change, accumulated J and K)."""
-    return 8 * nao * nao * n_dm * (3 + 5 + (4 if incremental else 0)) + 4 * nbas * nbas
+    the screening table and its copy per pair) for hermi = 1; incremental
+    mode keeps four more (the previous density, the density change,
+    accumulated J and K)."""
+    return (8 * nao * nao * n_dm * (3 + 5 + (4 if incremental else 0)) + 4 * nbas * nbas
+            + 2 * nbas * (nbas + 1))
 
 
 def table_bound(nbas: int) -> int:
-    """Upper estimate of a plan's pair tables before it exists: nbas^2/2
-    pairs of 40-byte records with 9 primitive pairs of 80 bytes each."""
-    return nbas * nbas // 2 * (40 + 9 * 80)
+    """Upper estimate of a plan's tables before it exists: every pair with its
+    two 64-byte records, its 16 bytes for the screening and a task row of 8
+    bytes for each of up to ten ket classes, and 9 primitive pairs of 80 bytes,
+    48 (FP32) and 72 (field-major); 256 KB for the tiles of the field-major
+    copy that a class does not fill (32 pairs of up to 36 primitive pairs in
+    (ss|, fewer in the others) and the build descriptors."""
+    return nbas * (nbas + 1) // 2 * (2 * 64 + 16 + 80 + 9 * (80 + 48 + 72)) + (1 << 18)
 
 
 def advance_density(d, sigma, gen):

@@ -82,3 +82,15 @@ def test_incremental_serving(torch):
             assert np.abs(mj - aj).max() <= ATOL
             assert np.abs(mk - ak).max() <= ATOL
             assert np.abs(mj - fj).max() <= 1e-9 and np.abs(mk - fk).max() <= 1e-9
+
+
+@pytest.mark.parametrize('basis', ['6-31g*', 'def2-svp', 'def2-tzvp'])
+@pytest.mark.parametrize('n', [1, 3, 12])
+def test_table_bound_holds(torch, basis, n):
+    """What admission reserves for a plan that does not exist yet is no less
+    than what the plan's tables take."""
+    from electrolites_b200 import clusters
+    from electrolites_b200.jk import VHFOpt
+    from electrolites_b200.serve import table_bound
+    mol = clusters.water_mole(n, 3.3 * n ** (1 / 3), 21, basis=basis)
+    assert VHFOpt(mol, 1e-13).build().memory()[0] <= table_bound(mol.nbas)
