@@ -1571,8 +1571,11 @@ static int plan_create(const int *atm, int natm, const int *bas, int nbas_user, 
     }
     // a pair of more than JK_PAIR_PRIMS primitive pairs goes on as several of
     // the same shells, its primitives dealt among them (integrals are linear in
-    // them): a warp's staged bra records then fit its share of shared memory
-    // whatever the contraction.  The parts follow the pairs.
+    // them): a warp's staged bra records (10 KB at most) then fit its share of
+    // shared memory whatever the contraction, in every form but the
+    // McMurchie-Davidson J kernels, which stage more per primitive and leave
+    // the classes that do not fit to the Rys J engine (jk_launch_class).  The
+    // parts follow the pairs.
     const size_t nwhole = cand.size();
     for (size_t c = 0; c < nwhole; ++c)
         if (cand[c].w > JK_PAIR_PRIMS) {

@@ -2011,6 +2011,15 @@ static int configure(K kern, int nt, size_t shm, KernelState &ks, const LaunchCf
     return 0;
 }
 
+// shared memory of the register form, FP32 records and tables not counted
+template <class C, int JX>
+static size_t reg_shm(const ClassArgs &a)
+{
+    const int hermite = JX == 3 ? JK_MD_DENS * md_nt(C::LI + C::LJ) : 0;   // per bra primitive
+    return (rys_smem_doubles<C, JX>() +
+            (size_t)(reg_threads<C>() / 32) * a.max_bra_prim * (JK_PRIM_STRIDE + hermite)) * sizeof(double);
+}
+
 // TEAMF: the team form (of a class that may also have the register form)
 template <class C, int NV, int OP, int JX = 0, bool TEAMF = !C::REG>
 static int launch_nv(const ClassArgs &a, const PlanView *views, const LaunchCfg &cfg, const char *tag,
@@ -2024,13 +2033,8 @@ static int launch_nv(const ClassArgs &a, const PlanView *views, const LaunchCfg 
     if constexpr (!TEAMF) {
         constexpr int NT = reg_threads<C>();
         auto kern = jk_reg_kernel<C, NT, NV, OP, JX>;
-        shm = (size_t)rys_smem_doubles<C, JX>() * sizeof(double) +
-              (size_t)(NT / 32) * a.max_bra_prim * JK_PRIM_STRIDE * sizeof(double);
-        if constexpr (JX == 3) {
-            shm += (size_t)(NT / 32) * a.max_bra_prim * JK_MD_DENS * md_nt(C::LI + C::LJ) *
-                   sizeof(double);
-            prm.a.mixed = 0;
-        }
+        shm = reg_shm<C, JX>(a);
+        if constexpr (JX == 3) prm.a.mixed = 0;
         prm.a.mixed_tab = 0;
         if (prm.a.mixed) {
             // the FP32 bra records, and the FP32 Rys table when the class keeps
@@ -2110,7 +2114,19 @@ int jk_launch_class(const ClassArgs &a, const PlanView *views, const LaunchCfg &
                 return (int)cudaErrorInvalidValue;
             }
             if (a.jx == 3) {
-                if constexpr (md_class<C>()) return launch_nv<C, 1, 1, 3>(a, views, cfg, tag, ks[6]);
+                if constexpr (md_class<C>()) {
+                    // the bra's Hermite densities of many primitives may not fit
+                    // ((pp|pp): about 99 primitive pairs, (ff|ss): 16): the Rys J
+                    // engine, whose x-space densities every such build has
+                    int most = 0;
+                    const cudaError_t e =
+                        cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, cfg.device);
+                    if (e != cudaSuccess) return (int)e;
+                    const size_t queue = reg_threads<C>() / 32 * 64 * sizeof(int);
+                    if (reg_shm<C, 3>(a) + queue > (size_t)most)
+                        return launch_nv<C, 1, 1, 2>(a, views, cfg, tag, ks[4]);
+                    return launch_nv<C, 1, 1, 3>(a, views, cfg, tag, ks[6]);
+                }
                 if (cfg.msg) snprintf(cfg.msg, 256, "class %s: no McMurchie-Davidson J kernel", tag);
                 return (int)cudaErrorInvalidValue;
             }

@@ -251,3 +251,62 @@ def test_builds_of_many_streams_and_threads(torch):
     for t in threads:
         t.join()
     assert not bad
+
+
+def _split_mol():
+    """s and d shells of twelve primitives: their pairs have 144 primitive
+    pairs and the plan splits them; a second atom of ordinary shells."""
+    prims = [(0.15 * 1.7 ** k, 1.0 / (k + 1)) for k in range(12)]
+    basis = {'H': [[0] + prims, [2] + prims], 'He': [[0, (0.9, 0.5), (0.3, 0.5)], [1, (0.7, 1.0)]]}
+    return Mole([('H', (0.0, 0.1, -0.2)), ('He', (0.8, -0.5, 0.9))], basis=basis, cart=True)
+
+
+def test_split_pairs_in_every_build(torch, oracle):
+    """J/K with symmetric and general densities, J alone by the J engine, the
+    (ij|kl) digest and the McMurchie-Davidson kernels (which leave classes of so
+    many primitives to the J engine), a batch, a mixed build, an allocation-free
+    build and a gradient, all with pairs that the plan splits."""
+    import ctypes
+
+    from electrolites_b200 import _lib
+    from electrolites_b200.batch import JKBatch
+    from electrolites_b200.jk import VHFOpt
+    mol = _split_mol()
+    n = mol.nao_cart
+    rng = np.random.default_rng(8)
+    gen = 0.3 * rng.standard_normal((2, n, n))
+    dms = gen + gen.transpose(0, 2, 1)
+    _check(torch, oracle, mol, dms, 1)
+    _check(torch, oracle, mol, gen, 0)
+    rj, rk, _ = oracle.jk(mol, dms, tol=TOL)
+    opt = VHFOpt(mol, TOL).build()
+    d = torch.as_tensor(dms, device='cuda')
+
+    def same(v, ref):
+        assert float(np.abs(v.cpu().numpy() - ref).max()) <= ATOL
+
+    same(opt.get_j(d), rj)
+    opt.set_jmd(1)
+    same(opt.get_j(d), rj)
+    opt.set_jmd(-1)
+    opt.set_jengine(False)
+    same(opt.get_j(d), rj)
+    opt.set_jengine(True)
+    water = VHFOpt(clusters.water_mole(1, 3.0, 7), TOL).build()
+    wd = torch.as_tensor(clusters.atomic_density(water.mol, 3)[None], device='cuda')
+    vj, vk = JKBatch().build([water, opt], [wd, d], 1)
+    same(vj[1], rj)
+    same(vk[1], rk)
+    mj, mk = (v.cpu().numpy() for v in opt.get_jk(d, 1, mixed_threshold=1e-6))
+    for m, r in ((mj, rj), (mk, rk)):
+        assert abs(np.einsum('nij,nji->', dms, m - r)) <= 1e-7
+    vj, vk = torch.empty_like(d), torch.empty_like(d)
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    _lib.check(_lib.lib().jk_build_noalloc(opt.plan, d.data_ptr(), 2, 1, 1, 1, vj.data_ptr(),
+                                           vk.data_ptr(), 0.0, st), 'jk_build_noalloc')
+    opt.sync()
+    same(vj, rj)
+    same(vk, rk)
+    got = VHFOpt(mol, 1e-16).build().jk_energy_per_atom(d, 1.0, 0.2).cpu().numpy()
+    ref, _ = oracle.grad_jk_fast(mol, dms, 1.0, 0.2, tol=0)
+    assert np.abs(got - ref).max() <= 1e-10 * np.abs(ref).max()
