@@ -1408,6 +1408,27 @@ struct TeamLayout {
     static constexpr int SIZE = ((E + ESZ) + 1) & ~1;
 };
 
+// sum over (a, b), a < NA, b < NB, of g[a GA + b GB] D[a da + b db], D in global
+// memory: the loop over a stays a loop.  The steps are run-time values (the
+// plan's AO order), so the unrolled loops formed a 64-bit address per element
+// and held them all: up to 3 KB of spills per thread in teams of up to 32 lanes,
+// 4 to 18 KB in larger ones and 40 in (ff|ff), where none, up to 1.3 KB and 6.5
+// are left ((ff|fd) of batches 2.4).  (H2O)_8 def2-TZVP with three
+// non-symmetric densities 50.6 -> 36.2 ms, eight symmetric ones of (H2O)_6
+// 21.4 -> 15.7, a mixed batch of 16 clusters of up to six 73.7 -> 62.9.
+template <int NA, int NB, int GA, int GB>
+__device__ __forceinline__ double block_dot(const double *g, const double *__restrict__ D, size_t da, int db)
+{
+    double s = 0.;
+#pragma unroll 1
+    for (int a = 0; a < NA; ++a) {
+#pragma unroll
+        for (int b = 0; b < NB; ++b) s = fma(g[a * GA + b * GB], __ldg(D + b * db), s);
+        D += da;
+    }
+    return s;
+}
+
 // digestion of a quartet held in shared memory, g[(i*NJ + j)*SQ + k*NL + l],
 // spread over the lanes of a team: one atomic per J/K element per quartet
 template <class C>
@@ -1416,30 +1437,21 @@ __device__ __forceinline__ void digest_shared(const PlanView &V, const double *g
                                               bool doK)
 {
     constexpr int NI = C::NI, NJ = C::NJ, NK = C::NK, NL = C::NL, NKL = NK * NL;
-    constexpr int SQ = TeamLayout<C>::SQ;
+    constexpr int SQ = TeamLayout<C>::SQ, SI = NJ * SQ;
     const AoIndex<C> ax(V);
     const size_t nao2 = ax.nao * ax.nao;
     for (int d = 0; d < (doJ ? V.n_j : 0); ++d) {
         const double *ds = V.dsJ + d * nao2;
         double *jh = V.Jh + d * nao2;
         for (int o = tl; o < NKL + NI * NJ; o += C::TEAM) {
-            double s = 0.;
             if (o < NKL) {
                 const int k = o / NL, l = o - (o / NL) * NL;
-#pragma unroll
-                for (int i = 0; i < NI; ++i)
-#pragma unroll
-                    for (int j = 0; j < NJ; ++j)
-                        s = fma(g[(i * NJ + j) * SQ + o], __ldg(ds + ax(i0, i, ax.in, j0, j, ax.j)), s);
-                atomicAdd(jh + ax(k0, k, ax.kn, l0, l, ax.l), s);
+                atomicAdd(jh + ax(k0, k, ax.kn, l0, l, ax.l),
+                          block_dot<NI, NJ, SI, SQ>(g + o, ds + ax(i0, 0, 0, j0, 0, 0), ax.in, ax.j));
             } else {
                 const int ij = o - NKL, i = ij / NJ, j = ij - (ij / NJ) * NJ;
-#pragma unroll
-                for (int k = 0; k < NK; ++k)
-#pragma unroll
-                    for (int l = 0; l < NL; ++l)
-                        s = fma(g[ij * SQ + k * NL + l], __ldg(ds + ax(k0, k, ax.kn, l0, l, ax.l)), s);
-                atomicAdd(jh + ax(i0, i, ax.in, j0, j, ax.j), s);
+                atomicAdd(jh + ax(i0, i, ax.in, j0, j, ax.j),
+                          block_dot<NK, NL, NL, 1>(g + ij * SQ, ds + ax(k0, 0, 0, l0, 0, 0), ax.kn, ax.l));
             }
         }
     }
@@ -1448,39 +1460,22 @@ __device__ __forceinline__ void digest_shared(const PlanView &V, const double *g
         const double *D = kdens(V, d, nao2);
         double *kh = V.Kh + d * nao2;
         for (int o = tl; o < N1 + N2 + N3 + N4; o += C::TEAM) {
-            double s = 0.;
             if (o < N1) {              // K_h[i,k] += sum_jl g D[j,l]
                 const int i = o / NK, k = o - (o / NK) * NK;
-#pragma unroll
-                for (int j = 0; j < NJ; ++j)
-#pragma unroll
-                    for (int l = 0; l < NL; ++l)
-                        s = fma(g[(i * NJ + j) * SQ + k * NL + l], __ldg(D + ax(j0, j, ax.jn, l0, l, ax.l)), s);
-                atomicAdd(kh + ax(i0, i, ax.in, k0, k, ax.k), s);
+                atomicAdd(kh + ax(i0, i, ax.in, k0, k, ax.k),
+                          block_dot<NJ, NL, SQ, 1>(g + i * SI + k * NL, D + ax(j0, 0, 0, l0, 0, 0), ax.jn, ax.l));
             } else if (o < N1 + N2) {  // K_h[i,l] += sum_jk g D[j,k]
                 const int t = o - N1, i = t / NL, l = t - (t / NL) * NL;
-#pragma unroll
-                for (int j = 0; j < NJ; ++j)
-#pragma unroll
-                    for (int k = 0; k < NK; ++k)
-                        s = fma(g[(i * NJ + j) * SQ + k * NL + l], __ldg(D + ax(j0, j, ax.jn, k0, k, ax.k)), s);
-                atomicAdd(kh + ax(i0, i, ax.in, l0, l, ax.l), s);
+                atomicAdd(kh + ax(i0, i, ax.in, l0, l, ax.l),
+                          block_dot<NJ, NK, SQ, NL>(g + i * SI + l, D + ax(j0, 0, 0, k0, 0, 0), ax.jn, ax.k));
             } else if (o < N1 + N2 + N3) {  // K_h[j,k] += sum_il g D[i,l]
                 const int t = o - N1 - N2, j = t / NK, k = t - (t / NK) * NK;
-#pragma unroll
-                for (int i = 0; i < NI; ++i)
-#pragma unroll
-                    for (int l = 0; l < NL; ++l)
-                        s = fma(g[(i * NJ + j) * SQ + k * NL + l], __ldg(D + ax(i0, i, ax.in, l0, l, ax.l)), s);
-                atomicAdd(kh + ax(j0, j, ax.jn, k0, k, ax.k), s);
+                atomicAdd(kh + ax(j0, j, ax.jn, k0, k, ax.k),
+                          block_dot<NI, NL, SI, 1>(g + j * SQ + k * NL, D + ax(i0, 0, 0, l0, 0, 0), ax.in, ax.l));
             } else {                   // K_h[j,l] += sum_ik g D[i,k]
                 const int t = o - N1 - N2 - N3, j = t / NL, l = t - (t / NL) * NL;
-#pragma unroll
-                for (int i = 0; i < NI; ++i)
-#pragma unroll
-                    for (int k = 0; k < NK; ++k)
-                        s = fma(g[(i * NJ + j) * SQ + k * NL + l], __ldg(D + ax(i0, i, ax.in, k0, k, ax.k)), s);
-                atomicAdd(kh + ax(j0, j, ax.jn, l0, l, ax.l), s);
+                atomicAdd(kh + ax(j0, j, ax.jn, l0, l, ax.l),
+                          block_dot<NI, NK, SI, NL>(g + j * SQ + l, D + ax(i0, 0, 0, k0, 0, 0), ax.in, ax.k));
             }
         }
     }
@@ -1758,9 +1753,10 @@ __device__ __forceinline__ bool team_one(const ClassArgs &A, const PlanView &V, 
 template <class C>
 constexpr int team_min_blocks()
 {
-    // (4 and 3 for the teams of 64 lanes and more, measured on (H2O)_13 def2-TZVP
-    // UHF: 47.4 -> 46.8 ms with smaller teams at 5, which cost (H2O)_2 def2-SVP
-    // 6% and stay at 3)
+    // (teams of 64 lanes and more at 3 and 2 lose 0.5 to 6% on def2-TZVP: (H2O)_5
+    // four non-symmetric densities 11.4 -> 12.0 ms, a batch of 40 clusters of up
+    // to two 7.1 -> 7.4, (H2O)_13 UHF 42.3 -> 42.6; smaller teams at 5 cost
+    // (H2O)_2 def2-SVP 6% and stay at 3)
     return C::TEAM <= 32 ? 3 : (C::TEAM <= 64 ? 4 : 3);
 }
 

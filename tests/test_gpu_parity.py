@@ -470,3 +470,22 @@ def test_reciprocal_square_root(torch):
     torch.cuda.synchronize()
     assert float((y / torch.rsqrt(x) - 1).abs().max()) <= 4.2 * u
     assert float((z / (1.0 / x) - 1).abs().max()) <= 3.2 * u
+
+
+@pytest.mark.parametrize('n_dm,hermi', [(1, 1), (3, 0), (6, 1), (7, 0)])
+def test_team_digest_of_many_densities(torch, oracle, n_dm, hermi):
+    """Every class with as many K densities as the team form stages in shared
+    memory and with more, which it reads in place, alone and in a batch (which
+    digests J from (ij|kl) too)."""
+    from electrolites_b200.batch import JKBatch
+    from electrolites_b200.jk import VHFOpt
+    mol = all_class_mol()
+    dms = densities(mol, 'random', n_dm, hermi, np.random.default_rng(n_dm))
+    rj, rk, _ = oracle.jk(mol, dms, tol=TOL)
+    opt = VHFOpt(mol, TOL).build()
+    d = torch.as_tensor(dms, device='cuda')
+    one = opt.get_jk(d, hermi)
+    vj, vk = JKBatch().build([opt, opt], [d, d], hermi)
+    for j, k in (one, (vj[0], vk[0]), (vj[1], vk[1])):
+        assert float(np.abs(j.cpu().numpy() - rj).max()) <= ATOL
+        assert float(np.abs(k.cpu().numpy() - rk).max()) <= ATOL

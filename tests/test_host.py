@@ -92,6 +92,23 @@ def test_a_destroyed_plan_frees_every_device_table():
         assert f'cudaFree(p->{t});' in free, t
 
 
+def test_small_team_kernels_do_not_spill():
+    """The compiler's report of the last build: the J/K team kernels of blocks
+    of 128 threads at 168 registers (teams of up to 32 lanes) hold everything in
+    registers.  (Addresses of unrolled density loads once took kilobytes.)"""
+    out = os.path.join(ROOT, 'electrolites_b200', 'csrc', '_build')
+    seen = 0
+    for tag in ('2121', '2221', '2222', '3111', '3121', '3130', '3131'):
+        path = os.path.join(out, f'class_{tag}.ptxas.txt')
+        if not os.path.exists(path):
+            pytest.skip('no compiler reports of a build')
+        for m in re.finditer(r'Function properties for (\S*jk_team_kernel\S*)\n.*?, (\d+) bytes spill stores',
+                             open(path).read()):
+            seen += 1
+            assert int(m.group(2)) == 0, m.group(1)
+    assert seen == 14
+
+
 def test_library_errors_without_device_or_bad_args():
     """Argument errors come back as codes with a message; no silent path."""
     from electrolites_b200 import _lib
