@@ -6,7 +6,9 @@ more, smaller tasks balance the persistent grid better, fewer, larger ones
 stage fewer bra pairs and claim fewer tasks -- a cap on resident blocks per
 SM, and whether mixed-precision builds run the class's low-bound quartets
 in FP32 (the per-class tuned threshold of the mixed form: a class where FP32
-measures slower keeps FP64).  The tuner times every candidate setting on a
+measures slower keeps FP64, one where both measure within 1% its default).
+Classes that the tuner's workloads do not hold (f shells) are not in the table
+and keep their defaults, which the code generator states.  The tuner times every candidate setting on a
 workload, all classes at once with per-class CUDA-event times, keeps the
 fastest setting of each class, and stores the table as JSON keyed by device
 name and form
@@ -74,7 +76,7 @@ def tune(target, run, run_mixed=None, reps: int = 2, candidates=CANDIDATES) -> d
         for k in timed[1]:
             on, off = timed[1][k], timed[0].get(k, timed[1][k])
             if _key(k) in table:
-                table[_key(k)][2] = 1 if on < 0.99 * off else 0
+                table[_key(k)][2] = 1 if on < 0.99 * off else 0 if on > 1.01 * off else -1
     apply(target, table)
     return table
 

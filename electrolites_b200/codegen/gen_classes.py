@@ -45,6 +45,12 @@ REG_MAX = 100         # largest (e0|f0) block kept in one thread's registers
 # 2.37, (fs|dd) 0.58 -> 0.79).  Builds of few quartets run them in the team
 # form (PASS_MIN_QUARTETS in csrc/jk_api.cu), so both are compiled
 REG_PASSES = frozenset({'2111', '2220', '3021', '3120', '3210', '3310'})
+# classes whose mixed builds run low-bound quartets in FP32 by default: those
+# where it does not lose (FP32 in every class: (H2O)_96 6-31G* 246 ms, in none
+# 212; (H2O)_20 def2-TZVP 54.2 / 44.6; a batch of 16 clusters of up to six in
+# def2-TZVP 62.6 ms with FP32 in every f class, 53.7 with these)
+FP32_DEFAULT = frozenset({'2020', '2222', '3222', '3320', '3321', '3322', '3330', '3331', '3332',
+                          '3333'})
 PASS_MAX = 80         # largest group of (e0|f0) elements of a pass
 FPART_MAX = 40        # f-components per warp in the team form
 LMAX = 3
@@ -728,12 +734,8 @@ def write_all(outdir, lmax=LMAX):
     reg.append('static const ClassEntry jk_class_table[JK_NCLASSES] = {')
     for A, B, cls in classes:
         form = 0 if cls.form == 'reg' else 1
-        # FP32 quartets by default in the register-form classes that run two
-        # blocks per SM ((e0|f0) block <= 27; in the larger register-form
-        # ones the second (FP32) copy of the quartet code costs more than it
-        # saves) and in the team form (FP32 2D integrals in shared memory)
         small = cls.ne * cls.nf <= REG_MAX
-        fp32 = 1 if (small and cls.ne * cls.nf <= 27) or not small else 0
+        fp32 = 1 if cls.tag in FP32_DEFAULT else 0
         # McMurchie-Davidson J kernel (J-only builds): register-form classes
         # up to JK_MD_LMAX; md_default: the classes where it measured faster
         # than the Rys J engine

@@ -85,6 +85,31 @@ def test_committed_table_is_well_formed():
                 assert v[0] > 0 and v[1] >= 0 and (len(v) < 3 or v[2] in (-1, 0, 1))
 
 
+def test_committed_table_holds_what_the_tuner_times():
+    """Its workloads are 6-31G*: the s, p and d classes and no others, so that
+    remaking the table loses no choice.  Classes outside it, on every device,
+    run FP32 quartets only where the generator says that they do not lose."""
+    from electrolites_b200 import autotune
+    from electrolites_b200.codegen import gen_classes
+    tags = {c.tag for _, _, c in gen_classes.all_classes()}
+    data = json.load(open(autotune.TABLE_PATH))
+    for entry in data.values():
+        for form in ('single', 'batch'):
+            assert set(entry[form]) == {t for t in tags if '3' not in t}
+    assert gen_classes.FP32_DEFAULT <= tags and len(gen_classes.FP32_DEFAULT) == 10
+
+
+def test_fp32_choice_within_one_percent_is_the_default(monkeypatch):
+    """Neither faster nor slower: the class keeps its default."""
+    from electrolites_b200 import autotune
+    keys = [(0, 0, 0, 0)]
+    monkeypatch.setattr(autotune, 'class_keys', lambda: keys)
+    t = FakeTarget(keys)
+    t.last_class_ms = lambda: ({keys[0]: 10.0 + 0.05 * (t.tune[0][2] == 1)}, 1)
+    table = autotune.tune(t, lambda: None, lambda: None, reps=1)
+    assert table['0000'][2] == -1
+
+
 class FakeJmd:
     """J-only per-class times: class 0 is faster with the MD kernel, class 1
     slower, class 2 has no MD kernel (set_jmd on it raises)."""
