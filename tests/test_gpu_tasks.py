@@ -310,3 +310,36 @@ def test_split_pairs_in_every_build(torch, oracle):
     got = VHFOpt(mol, 1e-16).build().jk_energy_per_atom(d, 1.0, 0.2).cpu().numpy()
     ref, _ = oracle.grad_jk_fast(mol, dms, 1.0, 0.2, tol=0)
     assert np.abs(got - ref).max() <= 1e-10 * np.abs(ref).max()
+
+
+class _Shifted:
+    """A molecule whose AOs start at the third row of its matrices."""
+
+    def __init__(self, mol):
+        self._mol = mol
+
+    def __getattr__(self, name):
+        return getattr(self._mol, name)
+
+    def ao_loc_nr(self, cart=True):
+        return np.asarray(self._mol.ao_loc_nr(cart=cart)) + 3
+
+
+@pytest.mark.parametrize('hermi', [1, 0])
+def test_ao_loc_that_starts_past_zero(torch, hermi):
+    """Rows before the first shell belong to no integral: their density is not
+    read, their J and K are zero, the rest is as without them."""
+    from electrolites_b200.jk import VHFOpt
+    mol = clusters.water_mole(2, 4.2, 9, basis='def2-svp')
+    n = mol.nao_cart
+    d = 0.2 * np.random.default_rng(2).standard_normal((2, n, n))
+    if hermi:
+        d = d + d.transpose(0, 2, 1)
+    big = np.full((2, n + 3, n + 3), 7.0)
+    big[:, 3:, 3:] = d
+    opt = VHFOpt(_Shifted(mol), TOL).build()
+    assert opt.nao == n + 3
+    ref = VHFOpt(mol, TOL).build().get_jk(torch.as_tensor(d), hermi)
+    for v, r in zip(opt.get_jk(torch.as_tensor(big), hermi), ref):
+        assert float((v[:, 3:, 3:] - r).abs().max()) <= ATOL
+        assert float(v[:, :3].abs().max()) == 0.0 and float(v[:, :, :3].abs().max()) == 0.0
