@@ -43,7 +43,9 @@ REG_MAX = 100         # largest (e0|f0) block kept in one thread's registers
 # 3.19 -> 1.33, (ff|ps) 2.20 -> 0.84; the next larger ones lose: (fp|pp)
 # 2.29 -> 3.15, (dp|dp) 1.60 -> 1.84, (dd|pp) 0.78 -> 1.29, (fp|fs) 1.73 ->
 # 2.37, (fs|dd) 0.58 -> 0.79).  Builds of few quartets run them in the team
-# form (PASS_MIN_QUARTETS in csrc/jk_api.cu), so both are compiled
+# form (PASS_MIN_QUARTETS in csrc/jk_api.cu), so both are compiled.  The passes
+# bound the accumulators; the whole bra-transferred and (ij|kl) blocks after them
+# spill (3.5 KB of stores per thread in (fd|ps) to 6.7 in (ff|ps))
 REG_PASSES = frozenset({'2111', '2220', '3021', '3120', '3210', '3310'})
 # classes whose mixed builds run low-bound quartets in FP32 by default: those
 # where it does not lose (FP32 in every class: (H2O)_96 6-31G* 246 ms, in none
@@ -482,13 +484,13 @@ MD_LMAX = 6              # = JK_MD_LMAX (csrc/jk_mdj.cuh)
 MD_DEFAULT = frozenset()
 
 # gradient forms: a quartet per lane for the classes of at most
-# GRAD_LANE_MAX integrals except GRAD_WARP, a warp per quartet for the rest.
-# Per-lane classes with more block products than GRAD_SPLIT_MIN accumulate a
-# group of at most GRAD_PASS_MAX block elements per pass over the primitives
-# (recurrences and roots recomputed per pass), so that the accumulators stay
-# in registers
+# GRAD_LANE_MAX integrals, a warp per quartet for the rest.  Per-lane classes
+# with more block products than GRAD_SPLIT_MIN accumulate a group of at most
+# GRAD_PASS_MAX block elements per pass over the primitives (recurrences and
+# roots recomputed per pass), which bounds what the primitive loops hold.  W, the
+# bra-transferred block and the shifted integrals around them are whole and
+# spill: 1 to 11 KB of stores per thread ((dp|ds) 10.6, (dd|ps) 9.9, (pp|pp) 5.2)
 GRAD_LANE_MAX = 108
-GRAD_WARP = frozenset()
 GRAD_SPLIT_MIN = 150
 GRAD_PASS_MAX = 64
 
@@ -512,8 +514,7 @@ def gen_grad_struct(cls):
     li, lj, lk, ll = cls.li, cls.lj, cls.lk, cls.ll
     lines = []
     rects = grad_rects(cls)
-    small = (ncart(li) * ncart(lj) * ncart(lk) * ncart(ll) <= GRAD_LANE_MAX
-             and cls.tag not in GRAD_WARP)
+    small = ncart(li) * ncart(lj) * ncart(lk) * ncart(ll) <= GRAD_LANE_MAX
     split = small and len(grad_members(cls)) > GRAD_SPLIT_MIN
     lines.append(f'    static constexpr bool G_SMALL = {"true" if small else "false"};')
     lines.append(f'    static constexpr bool G_SPLIT = {"true" if split else "false"};')

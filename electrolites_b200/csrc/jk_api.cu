@@ -207,7 +207,6 @@ struct Engine {
     // McMurchie-Davidson J may serve its classes: a J-only build of one plan,
     // the Coulomb operator, at most JK_MD_DENS densities
     bool md_ok = false;
-    bool jx_reg = true;             // J/K builds: register-form classes too
     double *jx_dens = nullptr, *jx_acc = nullptr;
     const jk_plan *jx_plan = nullptr;
     const double *jx_ds = nullptr;
@@ -934,12 +933,9 @@ static ClassArgs class_args(const Engine &E, int c, int l, const PlanView **host
     a.mixed_tab = 0;
     a.shard_rank = E.shard_rank;
     a.shard_size = E.shard_size;
-    // the J engine: every class of a J-only build; with K, the team-form
-    // classes (J from the x-space contraction, K from the transfers)
+    // the J engine: J from the x-space contraction, K (1) from the transfers
     // (2: a J-only build, whose register-form kernel has no K path)
-    a.jx = E.jx && (E.jx_jonly || jk_class_table[c].form == 1 || E.jx_reg)
-               ? (E.jx_jonly ? 2 : 1)
-               : 0;
+    a.jx = !E.jx ? 0 : E.jx_jonly ? 2 : 1;
     // 3: McMurchie-Davidson J in place of the J engine (the class's choice)
     if (a.jx == 2 && E.md_ok && jk_class_table[c].md && E.tune[c].jmd) a.jx = 3;
     a.team = E.cls_team[c];

@@ -160,7 +160,8 @@ struct ClassDesc {
     int tile0, ntiles;       // scan tiles of JK_ROW_TILE rows
     int target;              // tasks the task size aims at
     int unit, hi;            // task sizes (kets): multiples of unit, at most hi
-    int fill;                // register form: warps that fill the GPU (team form: 0)
+    int fill;                // tasks of a warp (register form, gradients, teams of
+                             // up to 32 lanes): warps that fill the GPU; else 0
     int cls;                 // class index (ClassDesc lists skip empty classes)
 };
 

@@ -20,16 +20,18 @@
 // per block in shared memory (molecules of up to JK_GRAD_SMEM_ATOMS atoms)
 // and added to the output once per block and atom component: every quartet
 // adds to the same natm x 3 numbers, so global atomics per quartet would all
-// contend for a few hundred addresses.  Two forms, chosen per class by
-// measurement in the code generator (G_SMALL):
+// contend for a few hundred addresses.  Two forms, by the number of integrals
+// of the class (G_SMALL, up to GRAD_LANE_MAX in the code generator):
 //   per lane: per quartet, primitive quartet and Rys root, the generated
 //   grad_root adds the root's 2D-integral products to four (e|f)-space
 //   blocks in registers: U (unweighted), RA, RB, RC (weighted by 2 alpha of
 //   the primitive of shell i, j, k); after the primitive sums the generated
 //   transfers of the shifted shells give each derivative block, which is
 //   contracted with W on the fly.  Classes with many block products
-//   (G_SPLIT) run one primitive pass per block so that one block is live at
-//   a time (four blocks spilled to local memory).  The bra atoms' forces add
+//   (G_SPLIT) run passes over the primitives, each for a group of f components
+//   of one block, so that their loops hold no more than a group; W, the
+//   transferred block and the shifted integrals of a shell are live together
+//   and still spill (1 to 11 KB per thread).  The bra atoms' forces add
 //   up in registers over a task; the ket shells' go to sums per ket pair;
 //   per warp (the larger classes): see grad_team_quartet below.
 #pragma once
@@ -863,8 +865,8 @@ constexpr size_t grad_team_doubles() { return C::G_SMALL ? 0 : (size_t)GradTeam<
 // ms, while (ps|ps) and (ds|ss) spill at that cap and lose, 4.2 -> 7.6 and
 // 3.9 -> 6.0 ms), the other per-lane kernels at 1 (255 registers); the
 // per-warp kernels at 3 (at most 170 registers; shared memory allows 3:
-// (dp|ds) 10.2 -> 8.8 ms, (dd|ps) 8.3 -> 7.5, (dp|pp) 8.2 -> 7.6), except
-// (dp|dp) and (fp|pp), which lose at 3 (6.8 -> 8.2, 59.7 -> 70.5 ms) and keep 1
+// (dp|pp) 8.2 -> 7.6 ms), except (dp|dp) and (fp|pp), which lose at 3 (6.8 ->
+// 8.2, 59.7 -> 70.5 ms) and keep 1
 template <class C>
 constexpr int grad_min_blocks()
 {
